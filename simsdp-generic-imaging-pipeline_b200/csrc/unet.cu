@@ -865,42 +865,43 @@ __global__ void __launch_bounds__(256) k_concat_up(int h, int w, int ca, int cb,
 }
 
 // ----------------------------------------------------------------------------
-// Weight gradient: dw[tap][o][i] += sum_p dz[p][o] * in[p + off(tap)][i], and
-// bias gradient db[o] += sum_p dz[p][o].
+// Weight gradient: dw[tap][o][i] += sum_p dz[p][o] * in[p + off(tap)][i].
 // One CTA: 32 output x 32 input channels, all 9 taps, over a strided set of
 // pixel tiles; per tile row one k16 step of m = output channel, n = input
-// channel, k = pixel.  A warp owns one row tap dy and half of the tile's rows:
-// the three column taps share its dz fragments, eight ldmatrix per 24 mma
-// (with a warp per tap it was four per eight: a quarter of the clocks each,
-// 46 clocks per SM and eight mma where the tensor pipe alone takes 17).
-// Partial sums are added to the FP32 gradients with atomics once per CTA.
-// The CTAs of the first input-channel block also sum the staged dz tile over
-// its pixels (the bias gradient; as kernels of their own those sums took
-// 625 us of a training step on 16 x 256^2).
+// channel, k = pixel.  A warp owns one row tap dy and 16 of the input
+// channels: the three column taps share its dz fragments, five ldmatrix per
+// twelve mma (with a warp per tap it was four per eight: a quarter of the
+// clocks each, 46 clocks per SM and eight mma where the tensor pipe alone
+// takes 17).  Partial sums are added to the FP32 gradients with atomics once
+// per CTA.
+// What is summed in one accumulator, and in which order, decides the rounding
+// of a gradient, and Adam turns the sign of a gradient near zero into a whole
+// step of the weight.  An accumulator therefore runs over all rows of its
+// tiles in order, and the number of CTAs per channel block is 4 per SM
+// whatever the kernel's occupancy: with the rows in two halves and another
+// number of CTAs the gradients of the 256-channel layer moved by 66 times what
+// two runs differ by.
 // A thread stages the same places of every tile, so that its offsets from
 // the tile's origin are computed once.
-// 16 x 256^2, all 14 layers: 2362 us with the bias sums -> 1607 us (32 -> 32
-// channels at level 0: 94 + 49 -> 87 us, 222 TFLOP/s; mma.sync alone reaches
-// 551).  Bound by latencies: the tensor pipe is 45 % busy with three warps
-// per scheduler, which the 96 accumulators a thread allow.
+// 16 x 256^2, all 14 layers: 1737 -> 1517 us (32 -> 32 channels at level 0
+// 94 -> 83 us, 232 TFLOP/s; mma.sync alone reaches 551).  Four CTAs per SM
+// hold one wave of most layers (three: 1619 us).
 // ----------------------------------------------------------------------------
 struct WgradArgs {
     const bf16 *dz;  // [n][h][w][cout]
     int cout;
     VIn in;
     float *dw;       // [9][cout][cin]
-    float *db;       // [cout]
     int n, tiles_x, tiles_y, ntiles;
 };
 
 constexpr int kWgDz = 4 * (kTH * kTW) * 16;  // dz tile: 4 planes x 128 pixels
 constexpr int kWgX = 4 * kHalo * 16;         // input halo: 4 planes x 180 pixels
 constexpr int kWgStage = kWgDz + kWgX;
-constexpr int kWgBytes = 2 * kWgStage;        // also holds the second half's 3 x 96 x 32 sums
-static_assert(kWgBytes >= 3 * 96 * 32 * 4, "partial sums in the staging buffers");
-constexpr int kWgThreads = 192;              // 3 row taps x 2 halves of the tile's rows
+constexpr int kWgBytes = 2 * kWgStage;
+constexpr int kWgThreads = 192;              // 3 row taps x 2 halves of the input channels
 
-__global__ void __launch_bounds__(kWgThreads, 2) k_wgrad3x3(WgradArgs p)
+__global__ void __launch_bounds__(kWgThreads, 4) k_wgrad3x3(WgradArgs p)
 {
     extern __shared__ __align__(128) unsigned char smem[];
     const int co0 = blockIdx.x * 32, ci0 = blockIdx.y * 32;
@@ -951,20 +952,16 @@ __global__ void __launch_bounds__(kWgThreads, 2) k_wgrad3x3(WgradArgs p)
         }
     };
 
-    float acc[3][2][4][4];  // column tap, output half, input octet
+    float acc[3][2][2][4];  // column tap, output half, input octet
 #pragma unroll
     for (int d = 0; d < 3; ++d)
 #pragma unroll
         for (int a = 0; a < 2; ++a)
 #pragma unroll
-            for (int b = 0; b < 4; ++b)
+            for (int b = 0; b < 2; ++b)
 #pragma unroll
                 for (int c = 0; c < 4; ++c) acc[d][a][b][c] = 0.f;
 
-    float bsum[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) bsum[e] = 0.f;
-    const bool bias = blockIdx.y == 0 && tid < 128;  // thread: plane tid / 32, pixels lane, lane + 32, ...
     int t = blockIdx.z;
     if (t < p.ntiles) {
         int tx = t % p.tiles_x, ty = (t / p.tiles_x) % p.tiles_y, img = t / (p.tiles_x * p.tiles_y);
@@ -994,17 +991,8 @@ __global__ void __launch_bounds__(kWgThreads, 2) k_wgrad3x3(WgradArgs p)
             __syncthreads();
             const unsigned char *base = smem + s * kWgStage;
             const uint32_t ds = smem_u32(base), xs = smem_u32(base + kWgDz);
-            if (bias) {
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    float f[8];
-                    unpack8(*reinterpret_cast<const uint4 *>(base + ((tid >> 5) * (kTH * kTW) + lane + 32 * k) * 16), f);
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) bsum[e] += f[e];
-                }
-            }
 #pragma unroll 1
-            for (int r = half * (kTH / 2); r < (half + 1) * (kTH / 2); ++r) {
+            for (int r = 0; r < kTH; ++r) {
                 uint32_t af[2][4];
 #pragma unroll
                 for (int mt = 0; mt < 2; ++mt) {
@@ -1014,58 +1002,63 @@ __global__ void __launch_bounds__(kWgThreads, 2) k_wgrad3x3(WgradArgs p)
                     ldsm4t(af[mt], ds + (pl * (kTH * kTW) + px) * 16);
                 }
 #pragma unroll
-                for (int dx = 0; dx < 3; ++dx)
+                for (int dx = 0; dx < 3; ++dx) {
+                    // transposed: matrix q = (pixel half q & 1, input plane 2 half + (q >> 1))
+                    uint32_t bfr[4];
+                    const int pl = 2 * half + (q >> 1);
+                    const int hidx = (r + dy) * kHW + (q & 1) * 8 + i8 + dx;
+                    ldsm4t(bfr, xs + (pl * kHalo + hidx) * 16);
 #pragma unroll
-                    for (int j = 0; j < 4; j += 2) {
-                        // transposed: matrix q = (pixel half q & 1, input plane j + (q >> 1))
-                        uint32_t bfr[4];
-                        const int pl = j + (q >> 1);
-                        const int hidx = (r + dy) * kHW + (q & 1) * 8 + i8 + dx;
-                        ldsm4t(bfr, xs + (pl * kHalo + hidx) * 16);
-#pragma unroll
-                        for (int mt = 0; mt < 2; ++mt) {
-                            mma16816(acc[dx][mt][j], af[mt], bfr[0], bfr[1]);
-                            mma16816(acc[dx][mt][j + 1], af[mt], bfr[2], bfr[3]);
-                        }
+                    for (int mt = 0; mt < 2; ++mt) {
+                        mma16816(acc[dx][mt][0], af[mt], bfr[0], bfr[1]);
+                        mma16816(acc[dx][mt][1], af[mt], bfr[2], bfr[3]);
                     }
+                }
             }
             __syncthreads();
         }
     }
-    // the two halves' sums: one set of atomics per CTA (same-address atomics
-    // of all CTAs queue up in L2)
-    float *part = reinterpret_cast<float *>(smem) + (dy * 96) * 32 + lane;
-    if (half) {
-#pragma unroll
-        for (int e = 0; e < 96; ++e) part[e * 32] = acc[e / 32][(e / 16) % 2][(e / 4) % 4][e % 4];
-    }
-    __syncthreads();
-    if (!half) {
-#pragma unroll
-        for (int e = 0; e < 96; ++e) acc[e / 32][(e / 16) % 2][(e / 4) % 4][e % 4] += part[e * 32];
-    }
     const int g = lane >> 2, tq = lane & 3;
-    if (!half) {
 #pragma unroll
-        for (int dx = 0; dx < 3; ++dx)
+    for (int dx = 0; dx < 3; ++dx)
 #pragma unroll
-            for (int mt = 0; mt < 2; ++mt)
+        for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
+            for (int j = 0; j < 2; ++j)
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int co = co0 + mt * 16 + g + (e >> 1) * 8;
-                        const int ci = ci0 + j * 8 + tq * 2 + (e & 1);
-                        atomicAdd(p.dw + ((size_t)(3 * dy + dx) * p.cout + co) * cin + ci, acc[dx][mt][j][e]);
-                    }
-    }
-    if (bias) {
+                for (int e = 0; e < 4; ++e) {
+                    const int co = co0 + mt * 16 + g + (e >> 1) * 8;
+                    const int ci = ci0 + half * 16 + j * 8 + tq * 2 + (e & 1);
+                    atomicAdd(p.dw + ((size_t)(3 * dy + dx) * p.cout + co) * cin + ci, acc[dx][mt][j][e]);
+                }
+}
+
+// Bias gradient: db[c] += sum_p dz[p][c]; c divides 256 (32 .. 256 channels).
+// A thread sums the pixels of its chain in order and adds the result with one
+// atomic, the composition the weight gradient's comment asks for: sums taken
+// from the weight gradient's tiles, or chains joined before the atomics, move
+// the biases by as much as two runs differ by.  Bound by the latency of a
+// chain's loads, so 32 pixels' are in flight together: all 14 layers of
+// 16 x 256^2 394 us (520 with 16; as the compiler unrolled it 622).
+constexpr int kBiasAhead = 32;
+__global__ void __launch_bounds__(256) k_bias_grad(const bf16 *__restrict__ dz, long long npix, int c,
+                                                  float *__restrict__ db)
+{
+    const int rows = 256 / c;
+    const int ch = threadIdx.x % c, r0 = threadIdx.x / c;
+    const long long first = (long long)blockIdx.x * rows + r0, step = (long long)gridDim.x * rows;
+    float s = 0.f;
+    for (long long p = first; p < npix; p += kBiasAhead * step) {
+        bf16 v[kBiasAhead];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            for (int o = 16; o > 0; o >>= 1) bsum[e] += __shfl_xor_sync(0xffffffffu, bsum[e], o);
-            if (lane == 0) atomicAdd(p.db + co0 + 8 * (tid >> 5) + e, bsum[e]);
+        for (int u = 0; u < kBiasAhead; ++u) {
+            const long long k = p + u * step;
+            v[u] = k < npix ? dz[k * c + ch] : __float2bfloat16_rn(0.f);
         }
+#pragma unroll
+        for (int u = 0; u < kBiasAhead; ++u) s += __bfloat162float(v[u]);
     }
+    atomicAdd(db + ch, s);
 }
 
 // ----------------------------------------------------------------------------
@@ -1200,7 +1193,10 @@ __global__ void k_head_fwd(long long npix, long long pix_per_img, int c, const b
 // dd0[p][c] = go[p] * bf16(hw[c]) * (d0[p][c] > 0); dhw[c] += sum_p go[p] d0[p][c];
 // dhb += sum_p go[p].  Four threads per pixel, eight channels each, so that
 // the sums stay in registers (one thread per pixel kept them in local
-// memory: 96 us for 16 x 256^2, now 29).
+// memory: 96 us for 16 x 256^2, now 36).  A warp takes 32 consecutive pixels
+// at a time; the chain of a pixel's place in the warp runs over all of the
+// warp's pixel groups, and the 32 chains are summed as a tree: over pixels 16
+// and 8 apart in the thread, then 4, 2 and 1 apart by shuffles.
 __global__ void __launch_bounds__(256) k_head_bwd(long long npix, const bf16 *__restrict__ d0,
                                                  const float *__restrict__ hw, const float *__restrict__ go,
                                                  bf16 *__restrict__ dd0, float *__restrict__ dhw,
@@ -1210,34 +1206,51 @@ __global__ void __launch_bounds__(256) k_head_bwd(long long npix, const bf16 *__
     __shared__ float s_dw[C + 1];
     for (int i = threadIdx.x; i <= C; i += blockDim.x) s_dw[i] = 0.f;
     __syncthreads();
-    const int g8 = threadIdx.x & 3;
-    float wv[8], part[8], pb = 0.f;
+    const int lane = threadIdx.x & 31, g8 = lane & 3;
+    float wv[8], part[4][8], pb[4];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-        wv[e] = __bfloat162float(__float2bfloat16_rn(hw[8 * g8 + e]));
-        part[e] = 0.f;
+    for (int e = 0; e < 8; ++e) wv[e] = __bfloat162float(__float2bfloat16_rn(hw[8 * g8 + e]));
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        pb[m] = 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) part[m][e] = 0.f;
     }
-    const long long stride = (long long)gridDim.x * (blockDim.x / 4);
-    for (long long p = (long long)blockIdx.x * (blockDim.x / 4) + (threadIdx.x >> 2); p < npix; p += stride) {
-        const float g = __ldg(go + p);
-        if (g8 == 0) pb += g;
-        float f[8], o[8];
-        unpack8(__ldg(reinterpret_cast<const uint4 *>(d0 + p * C + 8 * g8)), f);
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long p0 = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31) + (lane >> 2); p0 < npix; p0 += stride) {
+        float gm[4];
+        uint4 v[4];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            o[e] = (f[e] > 0.f) ? g * wv[e] : 0.f;
-            part[e] += g * f[e];
+        for (int m = 0; m < 4; ++m) {
+            const long long p = min(p0 + 8 * m, npix - 1);
+            gm[m] = __ldg(go + p);
+            v[m] = __ldg(reinterpret_cast<const uint4 *>(d0 + p * C + 8 * g8));
         }
-        *reinterpret_cast<uint4 *>(dd0 + p * C + 8 * g8) = pack8(o);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            const long long p = p0 + 8 * m;
+            if (p >= npix) continue;
+            const float g = gm[m];
+            pb[m] += g;
+            float f[8], o[8];
+            unpack8(v[m], f);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                o[e] = (f[e] > 0.f) ? g * wv[e] : 0.f;
+                part[m][e] += g * f[e];
+            }
+            *reinterpret_cast<uint4 *>(dd0 + p * C + 8 * g8) = pack8(o);
+        }
     }
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-        float v = part[e];
+        float v = (part[0][e] + part[2][e]) + (part[1][e] + part[3][e]);
         for (int off = 16; off >= 4; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-        if ((threadIdx.x & 31) < 4) atomicAdd(&s_dw[8 * g8 + e], v);
+        if (lane < 4) atomicAdd(&s_dw[8 * g8 + e], v);
     }
-    for (int off = 16; off; off >>= 1) pb += __shfl_xor_sync(0xffffffffu, pb, off);
-    if ((threadIdx.x & 31) == 0) atomicAdd(&s_dw[C], pb);
+    float b = (pb[0] + pb[2]) + (pb[1] + pb[3]);
+    for (int off = 16; off >= 4; off >>= 1) b += __shfl_xor_sync(0xffffffffu, b, off);
+    if (lane == 0) atomicAdd(&s_dw[C], b);
     __syncthreads();
     for (int k = threadIdx.x; k < C; k += blockDim.x) atomicAdd(dhw + k, s_dw[k]);
     if (threadIdx.x == 0) atomicAdd(dhb, s_dw[C]);
@@ -1621,20 +1634,11 @@ int wgrad(const bf16 *dz, int cout, VIn in, float *dw, float *db, int n, cudaStr
     a.ntiles = (int)tiles(n, in.h, in.w);
     const int cin = in.ca + in.cb;
     const int blocks_xy = (cout / 32) * (cin / 32);
-    // CTAs per channel block: the fewest tile times over whole waves of two
-    // CTAs per SM, a wave's start and its atomics counted as three tiles
-    int z = 1, best = 0x7fffffff;
-    for (int c = 1; c <= std::min(a.ntiles, 4 * num_sms()); ++c) {
-        const int waves = (c * blocks_xy + 2 * num_sms() - 1) / (2 * num_sms());
-        const int cost = waves * ((a.ntiles + c - 1) / c + 3);
-        if (cost < best) {
-            best = cost;
-            z = c;
-        }
-        if (waves > 4) break;
-    }
-    a.db = db;
+    const int z = std::max(1, std::min(a.ntiles, (4 * num_sms() + blocks_xy - 1) / blocks_xy));
     k_wgrad3x3<<<dim3(cout / 32, cin / 32, z), kWgThreads, kWgBytes, st>>>(a);
+    SDP_LAUNCH_CHECK();
+    const long long np = (long long)n * in.h * in.w;
+    k_bias_grad<<<grid_for(np / (256 / cout) + 1), 256, 0, st>>>(dz, np, cout, db);
     SDP_LAUNCH_CHECK();
     return SDP_OK;
 }
@@ -1972,7 +1976,7 @@ SDP_EXPORT int sdp_unet_backward(sdp_unet *u, const float *grad_output, void *st
     float *G = u->grad;
     const int c0 = ch(u, 0);
     // head: dZ(d0) -> gz[0][0]
-    k_head_bwd<<<std::min(grid_for(4 * np), 8 * num_sms()), 256, 0, st>>>(
+    k_head_bwd<<<grid_for(np), 256, 0, st>>>(
         np, u->d[0][1], u->master + u->head_off, grad_output, u->gz[0][0], G + u->head_off, G + u->head_off + c0);
     SDP_LAUNCH_CHECK();
     // decoder, top (level 0) down to level kLevels - 2; gz[l][0] holds dZ of d_l on entry
