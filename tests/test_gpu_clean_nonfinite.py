@@ -99,3 +99,20 @@ def test_equal_peaks(sdp, device, actors, oracle32, G):
     s = _compare(sdp, device, actors, oracle32, res, psf, 30)
     first = [(int(round(float(y) / 1e-5)) + G // 2, int(round(float(x) / 1e-5)) + G // 2) for x, y, _ in s[:len(spots)]]
     assert first == sorted(spots)
+
+
+def test_infinite_psf_max(sdp, device, actors, oracle32):
+    """An infinite PSF maximum: the scale is zero, zero times infinity a NaN
+    inside the component's window, and nothing changes outside it."""
+    res = _sky(2784, 6)
+    res[3, 5] = 2.0
+    _compare(sdp, device, actors, oracle32, res, _point_psf(2784), 1, psf_max=float("inf"))
+
+
+def test_negative_zeros(sdp, device, actors, oracle32):
+    """Zeros keep their sign outside a component's window, also under a
+    negative component (-0 - (-0) is +0)."""
+    res, psf = _sky(2784, 7), _point_psf(2784)
+    res[np.abs(res) < 0.01] = -0.0
+    res[5, 7] = -2.0
+    _compare(sdp, device, actors, oracle32, res, psf, 6)
