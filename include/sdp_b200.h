@@ -545,7 +545,9 @@ typedef struct sdp_clean_params {
  * *num_sources_dev is set to -1.  Larger images keep per-tile bounds and
  * touch only the tiles that can hold the maximum, also in one cooperative
  * launch, and a last pass brings the residual up to date; where noise_factor
- * x loop_gain >= 0.5 they use one launch per minor cycle. */
+ * x loop_gain >= 0.5, or the workspace is smaller than the size asked for this
+ * grid_size but not than the one for a grid_size above 16383, they use one
+ * launch per minor cycle.  A workspace below that size is refused. */
 int sdp_hogbom_workspace_bytes(int grid_size, size_t *bytes);
 int sdp_hogbom(const sdp_clean_params *p, float *residual_inout, const float *psf, float *model_inout,
                sdp_float3 *sources, int *num_sources_dev, void *workspace, size_t workspace_bytes, void *stream);
