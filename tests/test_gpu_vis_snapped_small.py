@@ -1,0 +1,58 @@
+"""Snapped gridding with half supports 1 and 2: a warp of the 16 x 16-tap kernel
+would hold one small box at a time, so these plans take the group kernels.
+Values against the oracle; time against the group kernels asked for by name
+(1.5 times for half support 1 when the plan took the other kernel)."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import synth
+from conftest import rel_rms
+
+pytestmark = pytest.mark.gpu
+
+
+def _plan(sdp, device, w, options=None):
+    import torch
+    uvw, gk, sup = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (w.uvw, w.gkernels, w.supports))
+    wk = sdp.Device.wkernels(gk, sup, w.supports)
+    return device.plan(w.cfg.grid_size, 16, w.cfg.uv_scale, w.cfg.w_scale, uvw, wk, wk, mode=sdp.SDP_GRID_SNAPPED,
+                       keep=(uvw, gk, sup), options=options)
+
+
+@pytest.mark.parametrize("supports", [[1] * 6, [2] * 6, [1, 2, 2, 1, 2, 1]])
+def test_values(sdp, device, oracle32, supports):
+    import torch
+    w = synth.make_workload("snap", 48, 800.0, "disc", 20, 256, 5, 0.05, 1.0, 1e-3, len(supports), supports,
+                            oversampling=16, seed=11)
+    vis, out = torch.from_numpy(w.vis).cuda(), torch.empty((256 * 256, 2), device="cuda")
+    plan = _plan(sdp, device, w)
+    plan.grid(vis, out)
+    torch.cuda.synchronize()
+    plan.check_flags()
+    plan.close()
+    ref = oracle32.gridding_cpu(256, 16, w.gkernels, w.supports, w.uvw, w.vis, w.cfg.uv_scale, w.cfg.w_scale)
+    assert rel_rms(out.cpu().numpy(), ref) <= 2e-6
+
+
+@pytest.mark.parametrize("hs", [1, 2])
+def test_no_slower_than_the_group_kernels(sdp, device, hs):
+    import torch
+    w = synth.make_workload("snap", 128, 5000.0, "disc", 40, 1024, 5, 0.05, 1.0, 1e-3, 8, [hs] * 8, oversampling=16, seed=3)
+    vis, out = torch.from_numpy(w.vis).cuda(), torch.empty((1024 * 1024, 2), device="cuda")
+    plans = {"default": _plan(sdp, device, w), "group": _plan(sdp, device, w, sdp.PlanOptions(16, 512, 8, 0))}
+    best = {}
+    for _ in range(5):
+        for name, plan in plans.items():
+            plan.grid(vis, out)
+            t0, t1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            t0.record()
+            for _ in range(20):
+                plan.grid(vis, out)
+            t1.record()
+            torch.cuda.synchronize()
+            best[name] = min(best.get(name, float("inf")), t0.elapsed_time(t1))
+    for plan in plans.values():
+        plan.close()
+    assert best["default"] <= 1.1 * best["group"], best
