@@ -31,10 +31,8 @@ struct sdp_visplan {
     int ntx, nty, nk, nbins, ntiles, hs_max, W, S;
     int tile = 16;                // uv tile side (grid cells)
     int chunk = 512;              // visibilities per work item (at most)
-    bool chunk_auto = true;       // no chunk asked for: small visibility sets are cut finer
-    int item = 512;               // visibilities per work item in use (at most chunk)
     int lanes = 0;                // lanes per visibility of the group kernels (0: warp-per-visibility kernel)
-    int warps = 4;                // warps per CTA of the warp-per-visibility kernel (0: by occupancy)
+    int warps = 4;                // warps per CTA of the warp-per-visibility kernel (0: by occupancy; 4: more for few visibilities)
     int pitch = 0;                // row pitch (float2) of the shared tiles: >= S, = 8 mod 16
     uint4 *geo = nullptr;         // plan order: packed tap-box geometry (fast path), see fast_geometry
     void *rec = nullptr;          // Rec<float> or Rec<double>

@@ -77,7 +77,7 @@ struct PlanDev {
     int *flags;
     const int *kdiff;  // bit 0: degridding set != gridding set; bit 1: != its conjugate
     int pitch;          // row pitch (float2) of the shared tiles of the warp-per-visibility kernels
-    int item;           // visibilities per work item (at most)
+    int chunk;          // visibilities per work item (at most)
     int qhs;            // half support of the visibilities with quad records (0: none)
     int snapped;        // snapped coordinates (inclusive taps, gridding_run.c:84-112)
     const uint4 *geo;   // packed tap-box geometry in plan order (see fast_geometry)
@@ -1659,15 +1659,15 @@ __global__ void __launch_bounds__(32 * NW, 20 / NW) k_vis_fast(PlanDev P, const 
                                                       const float2 *__restrict__ measured)
 {
     extern __shared__ __align__(16) unsigned char smem_fast[];
-    const size_t stage_b = fast_stage_bytes(P.item);
+    const size_t stage_b = fast_stage_bytes(P.chunk);
     int4 *planes = reinterpret_cast<int4 *>(smem_fast + stage_b);
     float2 *mtile = reinterpret_cast<float2 *>(smem_fast + stage_b + 16 * (size_t)P.nk_g);
     float2 *subs = mtile + (OP != OP_GRID ? (size_t)P.S * P.pitch : 0);
     __shared__ __align__(16) float s_wscr[NW * kFastVB * 5];
     __shared__ int s_item, s_fail;
     __shared__ __align__(8) uint64_t s_bar;
-    ItemStage stg{reinterpret_cast<uint4 *>(smem_fast), reinterpret_cast<uint4 *>(smem_fast + 16 * (size_t)P.item),
-                  reinterpret_cast<float2 *>(smem_fast + 32 * (size_t)P.item), &s_bar, 0u, &s_fail, &s_item};
+    ItemStage stg{reinterpret_cast<uint4 *>(smem_fast), reinterpret_cast<uint4 *>(smem_fast + 16 * (size_t)P.chunk),
+                  reinterpret_cast<float2 *>(smem_fast + 32 * (size_t)P.chunk), &s_bar, 0u, &s_fail, &s_item};
     if (threadIdx.x == 0) {
         s_fail = 0;
         s_item = atomicAdd(P.item_counter, 1);
@@ -1887,14 +1887,14 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_vis_wide(PlanDev P, const 
     constexpr bool kGrids = (OP != OP_DEGRID);
     constexpr bool kConv = (OP != OP_GRID);
     extern __shared__ __align__(16) unsigned char smem_fast[];
-    const size_t stage_b = wide_stage_bytes(P.item);
+    const size_t stage_b = wide_stage_bytes(P.chunk);
     int4 *planes = reinterpret_cast<int4 *>(smem_fast + stage_b);
     float2 *mtile = reinterpret_cast<float2 *>(smem_fast + stage_b + 16 * (size_t)P.nk_g);
     float2 *subs = mtile + (kConv ? (size_t)P.S * P.pitch : 0);
     __shared__ int s_item, s_fail;
     __shared__ __align__(8) uint64_t s_bar;
     ItemStage stg{reinterpret_cast<uint4 *>(smem_fast), nullptr,
-                  reinterpret_cast<float2 *>(smem_fast + 16 * (size_t)P.item), &s_bar, 0u, &s_fail, nullptr};
+                  reinterpret_cast<float2 *>(smem_fast + 16 * (size_t)P.chunk), &s_bar, 0u, &s_fail, nullptr};
     if (threadIdx.x == 0) {
         s_fail = 0;
         s_item = atomicAdd(P.item_counter, 1);
@@ -2269,7 +2269,7 @@ static PlanDev plan_dev(const sdp_visplan *p)
     d.item_counter = p->item_counter;
     d.flags = p->flags;
     d.pitch = p->pitch;
-    d.item = p->item;
+    d.chunk = p->chunk;
     d.qhs = p->hs_max <= 4 && p->mode == SDP_GRID_STD ? p->hs_max : 0;
     d.snapped = p->mode == SDP_GRID_SNAPPED ? 1 : 0;
     d.geo = p->geo;
@@ -2376,7 +2376,7 @@ static void plan_layout(const sdp_visplan *p, size_t *off, size_t *total)
     off[5] = o; o = align_up(o + sizeof(int) * ((size_t)p->nbins + 1), 256);              // offsets
     off[6] = o; o = align_up(o + sizeof(int) * ((size_t)p->ntiles + 1), 256);             // item counts
     off[7] = o; o = align_up(o + sizeof(int) * ((size_t)p->ntiles + 1), 256);             // item offsets
-    off[8] = o; o = align_up(o + sizeof(int4) * ((size_t)n / p->item + p->ntiles + 1), 256);// items
+    off[8] = o; o = align_up(o + sizeof(int4) * ((size_t)n / p->chunk + p->ntiles + 1), 256);// items
     off[9] = o; o = align_up(o + sizeof(int) * nb_scan, 256);                             // scan scratch
     off[10] = o; o = align_up(o + sizeof(int) * 4, 256);                                  // scalars
     off[11] = o; o = align_up(o + sizeof(float2) * (size_t)std::max(n, 1), 256);          // measured
@@ -2402,14 +2402,16 @@ size_t visplan_record_bytes(const sdp_visplan *p)
 }
 
 // Plans of the 16 x 16-tap kernel (k_vis_wide): half supports of 5 to 8, or
-// snapped coordinates (boxes of 2 hs + 1 taps) from a half support of 3 on.
-// It takes one visibility per warp whatever the box, the group kernels
-// several small ones: 325,120 snapped visibilities at 1024^2, half support
-// 1 / 2 / 3, 103 / 103 / 104 us against their 67 / 97 / 130.
+// snapped coordinates (boxes of 2 hs + 1 taps) from a half support of 3 on, and
+// below in few work items.  It takes one visibility per warp whatever the
+// box, the group kernels several small ones: snapped, half support 1 / 2 / 3,
+// 80,640 visibilities at 512^2 45 / 45 / 46 us against their 50 / 69 / 90, 325,120
+// at 1024^2 103 / 103 / 102 against 67 / 97 / 130.
 static bool wide_plan(const sdp_visplan *p)
 {
-    return p->lanes == 0 && p->hs_max <= 8 &&
-           ((p->mode == SDP_GRID_STD && p->hs_max > 4) || (p->mode == SDP_GRID_SNAPPED && p->hs_max > 2));
+    if (p->lanes != 0 || p->hs_max < 1 || p->hs_max > 8) return false;
+    if (p->mode == SDP_GRID_STD) return p->hs_max > 4;
+    return p->mode == SDP_GRID_SNAPPED && (p->hs_max > 2 || 2LL * (p->n / p->chunk) < 3 * num_sms());
 }
 
 int visplan_setup(sdp_visplan *p, const sdp_geometry *geom, const sdp_wkernels *gk, const sdp_wkernels *dk, int n,
@@ -2445,13 +2447,6 @@ int visplan_setup(sdp_visplan *p, const sdp_geometry *geom, const sdp_wkernels *
     p->pitch = p->S + ((8 - p->S % 16) + 16) % 16;
     // (the 16 x 16 kernel touches two rows of up to sixteen cells, conflict-free at any pitch)
     if (wide_plan(p)) p->pitch = p->S;
-    // Visibilities per work item.  The longest item bounds a pass over few
-    // visibilities, so that small sets are cut finer: about two items per
-    // resident CTA (148 SMs x 5), down to 64 visibilities (120,960 of half
-    // support 3 at 512^2: 92 us a pass with items of 512 and no quad records,
-    // 34 us with items of 96 and quad records)
-    p->item = p->chunk;
-    if (p->chunk_auto) p->item = std::min(p->chunk, std::max(64, (n / 1480 + 31) / 32 * 32));
     const int os = geom->oversampling;
     p->phase_major = (os & (os - 1)) == 0 ? 1 : 0;
     p->dinv_nc = 2 * (os + 1);
@@ -2506,7 +2501,7 @@ int visplan_kernels(sdp_visplan *p, cudaStream_t st)
             // conjugated copy of the degridding set: a w < 0 visibility's taps
             // read it, so the four-visibility path needs no sign per sample
             const long long nconj = (long long)p->dk_conj_off;
-            k_conj_copy<<<(int)std::min<long long>((nconj + 255) / 256, 148 * 16), 256, 0, st>>>(
+            k_conj_copy<<<(int)std::min<long long>((nconj + 255) / 256, num_sms() * 16), 256, 0, st>>>(
                 p->dk2, nconj, p->dk2 + nconj);
             SDP_LAUNCH_CHECK();
             const int ne = (int)plan_dinv_entries(p);
@@ -2610,17 +2605,17 @@ int visplan_build(sdp_visplan *p, void *arena, const float3 *uvw, cudaStream_t s
                                                                   p->gbase, p->dpoff, p->dk_conj_off, qhs);
         SDP_LAUNCH_CHECK();
     }
-    k_item_counts<<<(p->ntiles + 255) / 256, 256, 0, st>>>(offsets, p->ntiles, p->nk, p->item, item_counts);
+    k_item_counts<<<(p->ntiles + 255) / 256, 256, 0, st>>>(offsets, p->ntiles, p->nk, p->chunk, item_counts);
     SDP_LAUNCH_CHECK();
     SDP_TRY(exclusive_scan(item_counts, item_offsets, p->ntiles, scan_scratch, st));
-    k_item_fill<<<(p->ntiles + 255) / 256, 256, 0, st>>>(offsets, item_offsets, p->ntiles, p->nk, p->item,
+    k_item_fill<<<(p->ntiles + 255) / 256, 256, 0, st>>>(offsets, item_offsets, p->ntiles, p->nk, p->chunk,
                                                           p->items);
     SDP_LAUNCH_CHECK();
     SDP_CUDA_TRY(cudaMemcpyAsync(p->n_items, item_offsets + p->ntiles, sizeof(int), cudaMemcpyDeviceToDevice, st));
     if (n > 0) {
-        const int cap = n / p->item + p->ntiles + 1;  // the items region's capacity
+        const int cap = n / p->chunk + p->ntiles + 1;  // the items region's capacity
         if (qhs > 0)
-            k_batch_flags<<<dim3(std::min(cap, 148 * 16), (p->item / 4 + 127) / 128), 128, 0, st>>>(
+            k_batch_flags<<<dim3(std::min(cap, num_sms() * 16), (p->chunk / 4 + 127) / 128), 128, 0, st>>>(
                 p->items, p->n_items, cap, qhs, p->geo, p->gbase);
         SDP_LAUNCH_CHECK();
     }
@@ -2695,7 +2690,6 @@ SDP_EXPORT int sdp_visplan_create_opt(sdp_visplan **out, const sdp_geometry *geo
     sdp_visplan *p = new sdp_visplan();
     p->tile = tile;
     p->chunk = chunk;
-    p->chunk_auto = !(opt && opt->chunk);
     p->lanes = lanes;
     p->warps = warps;
     int status = visplan_setup(p, geom, gk, dk, num_vis, grid_mode);
@@ -2875,14 +2869,14 @@ static int launch_tiles_lg(sdp_visplan *p, int op, const float2 *vis_in, const f
 static bool fast_eligible(const sdp_visplan *p)
 {
     return p->mode == SDP_GRID_STD && p->lanes == 0 && p->hs_max >= 1 && p->hs_max <= 4 &&
-           fast_smem_bytes(OP_CYCLE_CONV, 4, p->S, p->pitch, p->gk.num_kernels, p->item) + kStaticSmem <= kSmemOptin;
+           fast_smem_bytes(OP_CYCLE_CONV, 4, p->S, p->pitch, p->gk.num_kernels, p->chunk) + kStaticSmem <= kSmemOptin;
 }
 
 template <typename T, int OP, int NW>
 static int launch_fast_nw(sdp_visplan *p, const float2 *vis_in, const float2 *in_grid, float2 *out_grid,
                           float2 *pred, float2 *delta, cudaStream_t st, int *resident_warps)
 {
-    const size_t smem = fast_smem_bytes(OP, NW, p->S, p->pitch, p->gk.num_kernels, p->item);
+    const size_t smem = fast_smem_bytes(OP, NW, p->S, p->pitch, p->gk.num_kernels, p->chunk);
     void (*fn)(PlanDev, const float2 *, const float2 *, float2 *, float2 *, float2 *, const float2 *) =
         p->hs_max == 4 ? k_vis_fast<T, OP, NW, 4> : k_vis_fast<T, OP, NW, 0>;
     if (smem + kStaticSmem > kSmemOptin) {
@@ -2917,6 +2911,22 @@ static int launch_fast_op(sdp_visplan *p, const float2 *vis_in, const float2 *in
         SDP_TRY((launch_fast_nw<T, OP, 4>(p, vis_in, in_grid, out_grid, pred, delta, st, &w4)));
         SDP_TRY((launch_fast_nw<T, OP, 8>(p, vis_in, in_grid, out_grid, pred, delta, st, &w8)));
         nw = (w4 > w8) ? 4 : 8;
+    } else if (nw == 4) {
+        // Few visibilities: the longest work item bounds the pass, so that more
+        // warps share one.  Fused pass, items of 512, 4 / 8 / 16 warps: 20,160
+        // visibilities at 256^2 60 / 39 / 26 us, 80,640 at 512^2 78 / 50 / 38,
+        // 161,280 82 / 54 / 53, 396,000 at 1024^2 96 / 83 / 100, 594,000 117 / 110 /
+        // 131.  (Items of 64 to 224 took as long, but put more partial sums
+        // through the grid's float atomics: 120,960 at 512^2, error 1.8e-7
+        // against 1.0e-7.)
+        const long long items = p->n / p->chunk;
+        int fit = 0;
+        if (2 * items < 3 * num_sms()) {
+            SDP_TRY((launch_fast_nw<T, OP, 16>(p, vis_in, in_grid, out_grid, pred, delta, st, &fit)));
+            if (fit) return launch_fast_nw<T, OP, 16>(p, vis_in, in_grid, out_grid, pred, delta, st, nullptr);
+        }
+        if (items < 5 * num_sms()) SDP_TRY((launch_fast_nw<T, OP, 8>(p, vis_in, in_grid, out_grid, pred, delta, st, &fit)));
+        if (fit) nw = 8;
     }
     if (nw == 4) return launch_fast_nw<T, OP, 4>(p, vis_in, in_grid, out_grid, pred, delta, st, nullptr);
     return launch_fast_nw<T, OP, 8>(p, vis_in, in_grid, out_grid, pred, delta, st, nullptr);
@@ -2941,7 +2951,7 @@ static int wide_warps(const sdp_visplan *p, int op)
     if (!wide_plan(p)) return 0;
     if (p->mode == SDP_GRID_SNAPPED ? op != OP_GRID : (op != OP_GRID && op != OP_DEGRID && op != OP_CYCLE_CONV)) return 0;
     for (int nw : {8, 4})
-        if (wide_smem_bytes(op, nw, p->S, p->pitch, p->gk.num_kernels, p->item) + kStaticSmem <= kSmemOptin) return nw;
+        if (wide_smem_bytes(op, nw, p->S, p->pitch, p->gk.num_kernels, p->chunk) + kStaticSmem <= kSmemOptin) return nw;
     return 0;
 }
 
@@ -2949,7 +2959,7 @@ template <typename T, int OP, int NW>
 static int launch_wide_nw(sdp_visplan *p, const float2 *vis_in, const float2 *in_grid, float2 *out_grid, float2 *pred,
                           float2 *delta, cudaStream_t st)
 {
-    const size_t smem = wide_smem_bytes(OP, NW, p->S, p->pitch, p->gk.num_kernels, p->item);
+    const size_t smem = wide_smem_bytes(OP, NW, p->S, p->pitch, p->gk.num_kernels, p->chunk);
     auto fn = k_vis_wide<T, OP, NW>;
     if (smem + kStaticSmem > 48 * 1024) SDP_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
@@ -3187,7 +3197,7 @@ SDP_EXPORT int sdp_visbatch_create(sdp_visbatch **out, sdp_visplan *const *plans
         b->hs_max = std::max(b->hs_max, p->hs_max);
         b->S_max = std::max(b->S_max, p->S);
         b->tile_f2 = std::max(b->tile_f2, (size_t)p->S * p->pitch);
-        b->chunk_max = std::max(b->chunk_max, p->item);
+        b->chunk_max = std::max(b->chunk_max, p->chunk);
         b->fast = b->fast && fast_eligible(p);
         b->hs4 = b->hs4 && p->hs_max == 4;
         if (b->fast && p->gbase) {
