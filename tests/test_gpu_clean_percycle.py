@@ -9,19 +9,31 @@ from __future__ import annotations
 import numpy as np
 import pytest
 
-from test_gpu_clean_deferred import _scene
-
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("G,noise,stops", [(2816, 5.1, False), (2816, 250.0, True), (2755, 5.1, False), (2755, 250.0, True)])
-def test_against_the_oracle(sdp, device, oracle32, G, noise, stops):
+def _scene(G):
+    """Eight peaks of 1 on noise of 0.01, a PSF of one pixel with sidelobes everywhere."""
+    rng = np.random.default_rng(G)
+    psf = (1e-4 * rng.standard_normal((G, G))).astype(np.float32)
+    psf[G // 2, G - G // 2] = 1.0  # the mirrored centre
+    res = (0.01 * rng.standard_normal((G, G))).astype(np.float32)
+    for y, x in rng.integers(0, G, (8, 2)):
+        res[y, x] = 1.0
+    return res.reshape(-1), psf.reshape(-1)
+
+
+# gain 0.5: the peaks go down by halves, and the mean of |r| is 0.008, so a
+# factor of 42 stops the loop between 0.25 and 0.125 (the oracle's running
+# mean in floats is off by some 0.2 %)
+@pytest.mark.parametrize("G", [2816, 2755])
+@pytest.mark.parametrize("noise,minor,stops", [(1.1, 60, False), (42.0, 200, True)])
+def test_against_the_oracle(sdp, device, oracle32, G, noise, minor, stops):
     import torch
-    minor = 200
-    res, psf = _scene(G, 8, 0.01, 2e-3, G)
-    n1, s1, m1, r1 = oracle32.hogbom(G, minor, minor, res, psf, 3.0, 1e-5, noise_factor=noise)
-    assert (10 < n1 < minor) if stops else n1 == minor
-    params = sdp.CleanParams(G, minor, minor, 0.1, noise, 0.0002, 3.0, 1e-5)
+    res, psf = _scene(G)
+    n1, s1, m1, r1 = oracle32.hogbom(G, minor, minor, res, psf, 3.0, 1e-5, loop_gain=0.5, noise_factor=noise)
+    assert n1 == (24 if stops else minor)
+    params = sdp.CleanParams(G, minor, minor, 0.5, noise, 0.0002, 3.0, 1e-5)
     r, p = torch.from_numpy(res.copy()).cuda(), torch.from_numpy(psf).cuda()
     m, s = torch.zeros(G * G, device="cuda"), torch.zeros((minor, 3), device="cuda")
     c = torch.zeros(1, dtype=torch.int32, device="cuda")
