@@ -12,9 +12,10 @@
 // global memory directly.  Row CTAs hold one or more whole rows.  Column CTAs
 // hold four adjacent columns (one 32-byte sector per row) of up to 2048
 // points, or eight of 1024 at 4096 and 8192 points; those columns are spread
-// over a cluster of Q CTAs: CTA c transforms the rows = c mod Q, and a radix-Q step over distributed shared
-// memory joins them.  (A CTA that held all of an 8192-point column had room
-// for one column: 8 bytes of every sector, 1290 us a pass.)
+// over a cluster of Q CTAs: CTA c transforms the rows = c mod Q, and a radix-Q
+// step over distributed shared memory joins them.  (A CTA that held all of an
+// 8192-point column had room for one column: 8 bytes of every sector, 1290 us
+// a pass.)
 // Row / column pass of the imaging transforms: 2048^2 10-12 / 18-19 us, 8192^2
 // 135-150 / 288-318 us (with full complex transforms 13-14 / 24-26 and
 // 225-238 / 450-494; the kernels before those 55 / 36 and 980 / 1290).  Rows
@@ -442,8 +443,8 @@ static std::mutex g_tw_mutex;
 static std::unordered_map<TwKey, float2 *, TwHash> g_tw;
 
 // Twiddle tables for size N on the current device (allocated on first use,
-// kept): exp(-2 pi i k / N), k < N, then the packed stage tables of a row and,
-// for N > 2^kColumnPoints, of a column part.
+// kept): exp(-2 pi i k / N), k < N, then the packed stage tables of a row and
+// of a column part.
 int fft_twiddles(int N, cudaStream_t st, const float2 **out)
 {
     int dev = 0;

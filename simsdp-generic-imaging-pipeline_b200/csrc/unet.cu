@@ -1257,10 +1257,9 @@ __global__ void __launch_bounds__(256) k_head_bwd(long long npix, const bf16 *__
 }
 
 // BF16 copies of all layers' FP32 weights, in one launch (blockIdx.y: the
-// layer; three launches per layer took 150 us of a training step,
-// this one 47): w[tap][o][i],
-// the data-gradient form wt[8 - tap][i][o], and both in the tensor-core
-// kernel's staging order (tc_index).
+// layer; three launches per layer took 150 us of a training step, this one
+// 47): w[tap][o][i], the data-gradient form wt[8 - tap][i][o], and both in the
+// tensor-core kernel's staging order (tc_index).
 struct LayerWeights {
     int cout, cin;
     const float *master;

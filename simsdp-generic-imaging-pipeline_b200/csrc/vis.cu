@@ -23,9 +23,10 @@
 // half support read one 16-byte quad record each (table bases, origin,
 // normalisation index) and reuse model reads and subgrid updates along runs
 // of one origin.  Plans of half supports 5 to 8 and snapped gridding take the
-// 16 x 16-tap variant (k_vis_wide).  The group kernels (k_tiles*, several visibilities per warp
-// on one shared subgrid) serve the rest: g2g, nearest-cell cycles, half
-// supports above 8 and batches of wide plans.
+// 16 x 16-tap variant (k_vis_wide).  The group kernels (k_tiles*, several
+// visibilities per warp on one shared subgrid) serve the rest: g2g,
+// nearest-cell cycles, half supports above 8, large snapped sets of half
+// supports 1 and 2, and batches of wide plans.
 #include <cstdio>
 #include <cstring>
 
@@ -2445,7 +2446,9 @@ int visplan_setup(sdp_visplan *p, const sdp_geometry *geom, const sdp_wkernels *
     // rows of 8-byte cells whose starts are 16 banks apart: the four rows a
     // warp touches in one access fall into two conflict-free bank halves
     p->pitch = p->S + ((8 - p->S % 16) + 16) % 16;
-    // (the 16 x 16 kernel touches two rows of up to sixteen cells, conflict-free at any pitch)
+    // (the 16 x 16 kernel touches two rows of up to sixteen cells, conflict-free
+    // at any pitch; its form for half supports up to 4, four rows of eight, is
+    // not where the pitch is a multiple of 16)
     if (wide_plan(p)) p->pitch = p->S;
     const int os = geom->oversampling;
     p->phase_major = (os & (os - 1)) == 0 ? 1 : 0;
@@ -2853,7 +2856,8 @@ static int launch_tiles_lg(sdp_visplan *p, int op, const float2 *vis_in, const f
     case OP_G2G: fn = k_tiles<T, SDP_GRID_STD, OP_G2G, LG>; break;
     default: return set_error(SDP_ERR_INVALID, "internal: op %d", op);
     }
-    if (smem + kStaticSmem > 48 * 1024) SDP_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem + kStaticSmem > 48 * 1024)
+        SDP_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     SDP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kThreads, smem));
     if (per_sm < 1) return set_error(SDP_ERR_RANGE, "tile kernel does not fit (%zu B shared memory)", smem);
@@ -2886,7 +2890,8 @@ static int launch_fast_nw(sdp_visplan *p, const float2 *vis_in, const float2 *in
         }
         return set_error(SDP_ERR_RANGE, "tile kernel does not fit (%zu B shared memory)", smem);
     }
-    if (smem + kStaticSmem > 48 * 1024) SDP_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem + kStaticSmem > 48 * 1024)
+        SDP_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     SDP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32 * NW, smem));
     if (resident_warps) {  // query only
@@ -2961,7 +2966,8 @@ static int launch_wide_nw(sdp_visplan *p, const float2 *vis_in, const float2 *in
 {
     const size_t smem = wide_smem_bytes(OP, NW, p->S, p->pitch, p->gk.num_kernels, p->chunk);
     auto fn = k_vis_wide<T, OP, NW>;
-    if (smem + kStaticSmem > 48 * 1024) SDP_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem + kStaticSmem > 48 * 1024)
+        SDP_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     SDP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32 * NW, smem));
     if (per_sm < 1) return set_error(SDP_ERR_RANGE, "tile kernel does not fit (%zu B shared memory)", smem);
@@ -3111,7 +3117,8 @@ static int launch_batch_lg(sdp_visbatch *b, int op, cudaStream_t st)
     void (*fn)(const PlanDev *, const BatchIO *, const int4 *, int, int *, int) =
         op == OP_CYCLE_CONV ? k_tiles_batch<T, SDP_GRID_STD, OP_CYCLE_CONV, LG>
                             : k_tiles_batch<T, SDP_GRID_STD, OP_CYCLE_NEAR, LG>;
-    if (smem + kStaticSmem > 48 * 1024) SDP_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem + kStaticSmem > 48 * 1024)
+        SDP_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     SDP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kThreads, smem));
     if (per_sm < 1) return set_error(SDP_ERR_RANGE, "batched tile kernel does not fit (%zu B shared memory)", smem);
@@ -3135,7 +3142,8 @@ static int launch_batch_fast_nw(sdp_visbatch *b, cudaStream_t st, int *resident_
         }
         return set_error(SDP_ERR_RANGE, "batched tile kernel does not fit (%zu B shared memory)", smem);
     }
-    if (smem + kStaticSmem > 48 * 1024) SDP_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem + kStaticSmem > 48 * 1024)
+        SDP_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     SDP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32 * NW, smem));
     if (resident_warps) {
