@@ -355,11 +355,11 @@ int sdp_visplan_destroy(sdp_visplan *plan);
  * 512), lanes per visibility (0: std_gridding plans with half supports up to
  * 4 take the warp-per-visibility kernel, one warp per visibility and a
  * private subgrid per warp, those up to 8 and snapped plans (from a half
- * support of 3, or of few visibilities) its 16 x 16-tap form, other plans the
- * fewest lanes their support needs; 8 / 16 / 32: the group kernels with that
+ * support of 3, or 2 and few visibilities) its 16 x 16-tap form, other plans
+ * the fewest lanes their support needs; 8 / 16 / 32: the group kernels with that
  * many lanes per visibility, several visibilities per warp on one shared
  * subgrid), warps per CTA of the warp-per-visibility kernel (0: by occupancy;
- * 8; or 4, which becomes 8 or 16 where there are fewer than 5 or 1.5 full work
+ * 8; or 4, which becomes 8 or 16 where there are fewer than 4 or 1.5 full work
  * items per SM).  Zero fields take the defaults.  sdp_visplan_create and the
  * actors use tile 16, items of 512, 4 warps.  Results are the same for every
  * shape up to the order of the floating-point sums. */

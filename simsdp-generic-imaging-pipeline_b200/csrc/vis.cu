@@ -25,8 +25,8 @@
 // of one origin.  Plans of half supports 5 to 8 and snapped gridding take the
 // 16 x 16-tap variant (k_vis_wide).  The group kernels (k_tiles*, several
 // visibilities per warp on one shared subgrid) serve the rest: g2g,
-// nearest-cell cycles, half supports above 8, large snapped sets of half
-// supports 1 and 2, and batches of wide plans.
+// nearest-cell cycles, half supports above 8, snapped sets of half support 1
+// and large ones of 2, and batches of wide plans.
 #include <cstdio>
 #include <cstring>
 
@@ -2404,15 +2404,17 @@ size_t visplan_record_bytes(const sdp_visplan *p)
 
 // Plans of the 16 x 16-tap kernel (k_vis_wide): half supports of 5 to 8, or
 // snapped coordinates (boxes of 2 hs + 1 taps) from a half support of 3 on, and
-// below in few work items.  It takes one visibility per warp whatever the
+// of 2 in few work items.  It takes one visibility per warp whatever the
 // box, the group kernels several small ones: snapped, half support 1 / 2 / 3,
-// 80,640 visibilities at 512^2 45 / 45 / 46 us against their 50 / 69 / 90, 325,120
-// at 1024^2 103 / 103 / 102 against 67 / 97 / 130.
+// 80,640 visibilities at 512^2, oversampling 16, 45 / 45 / 46 us against their
+// 50 / 69 / 90, oversampling 12 59 / 60 / 60 against 49 / 67 / 84; 325,120 at
+// 1024^2 103 / 103 / 102 against 67 / 97 / 130.
 static bool wide_plan(const sdp_visplan *p)
 {
     if (p->lanes != 0 || p->hs_max < 1 || p->hs_max > 8) return false;
     if (p->mode == SDP_GRID_STD) return p->hs_max > 4;
-    return p->mode == SDP_GRID_SNAPPED && (p->hs_max > 2 || 2LL * (p->n / p->chunk) < 3 * num_sms());
+    const bool few = 2LL * (p->n / p->chunk) < 3 * num_sms();
+    return p->mode == SDP_GRID_SNAPPED && (p->hs_max > 2 || (p->hs_max == 2 && few));
 }
 
 int visplan_setup(sdp_visplan *p, const sdp_geometry *geom, const sdp_wkernels *gk, const sdp_wkernels *dk, int n,
@@ -2920,8 +2922,8 @@ static int launch_fast_op(sdp_visplan *p, const float2 *vis_in, const float2 *in
         // Few visibilities: the longest work item bounds the pass, so that more
         // warps share one.  Fused pass, items of 512, 4 / 8 / 16 warps: 20,160
         // visibilities at 256^2 60 / 39 / 26 us, 80,640 at 512^2 78 / 50 / 38,
-        // 161,280 82 / 54 / 53, 396,000 at 1024^2 96 / 83 / 100, 594,000 117 / 110 /
-        // 131.  (Items of 64 to 224 took as long, but put more partial sums
+        // 161,280 82 / 54 / 53, 241,920 96 / 60 / 67; 325,120 at 1024^2 68 / 71 / -,
+        // 396,000 96 / 83 / 100.  (Items of 64 to 224 took as long, but put more partial sums
         // through the grid's float atomics: 120,960 at 512^2, error 1.8e-7
         // against 1.0e-7.)
         const long long items = p->n / p->chunk;
@@ -2930,7 +2932,7 @@ static int launch_fast_op(sdp_visplan *p, const float2 *vis_in, const float2 *in
             SDP_TRY((launch_fast_nw<T, OP, 16>(p, vis_in, in_grid, out_grid, pred, delta, st, &fit)));
             if (fit) return launch_fast_nw<T, OP, 16>(p, vis_in, in_grid, out_grid, pred, delta, st, nullptr);
         }
-        if (items < 5 * num_sms()) SDP_TRY((launch_fast_nw<T, OP, 8>(p, vis_in, in_grid, out_grid, pred, delta, st, &fit)));
+        if (items < 4 * num_sms()) SDP_TRY((launch_fast_nw<T, OP, 8>(p, vis_in, in_grid, out_grid, pred, delta, st, &fit)));
         if (fit) nw = 8;
     }
     if (nw == 4) return launch_fast_nw<T, OP, 4>(p, vis_in, in_grid, out_grid, pred, delta, st, nullptr);

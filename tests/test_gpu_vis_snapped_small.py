@@ -1,5 +1,6 @@
 """Snapped gridding with half supports 1 and 2: a warp of the 16 x 16-tap kernel
-would hold one small box at a time, so these plans take the group kernels.
+would hold one small box at a time, so these plans take the group kernels (half
+support 2 from 1.5 full work items per SM on).
 Values against the oracle; time against the group kernels asked for by name
 (1.5 times for half support 1 when the plan took the other kernel)."""
 from __future__ import annotations

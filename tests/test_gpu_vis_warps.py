@@ -42,6 +42,7 @@ def _plan(sdp, device, w, tables, options=None):
     (20, 3, 16, 512, False), (20, 4, 16, 512, False),  # 44 full items: 16 warps
     (20, 4, 16, 64, False), (20, 2, 16, 64, True),     # 352: 8 warps
     (48, 4, 16, 64, False), (48, 3, 16, 64, False),    # 846: 4 warps
+    (20, 3, 16, 512, True),                            # 16 warps, FP64 coordinates
     (20, 4, 32, 512, False), (20, 4, 48, 512, True)])  # 16 subgrids do not fit; nor do 8
 def test_values(sdp, device, oracle32, oracle64, n_time, hs, tile, chunk, f64):
     import torch
