@@ -60,7 +60,7 @@ __device__ __forceinline__ void phase_sincos(double u, double v, double w, doubl
 template <bool FAST>
 __device__ __forceinline__ void dft_tile(const SrcTerm *tile, int cnt, double u, double v, double w, float &sx, float &sy)
 {
-#pragma unroll 4
+#pragma unroll (FAST ? 4 : 8)
     for (int k = 0; k < cnt; ++k) {
         const SrcTerm t = tile[k];
         float s, c;
@@ -128,7 +128,7 @@ template <bool FAST>
 __device__ __forceinline__ void gauss_tile(const SrcTermG *tile, int cnt, double u, double v, double w, float q, float &sx,
                                            float &sy)
 {
-#pragma unroll 4
+#pragma unroll (FAST ? 4 : 8)
     for (int k = 0; k < cnt; ++k) {
         const SrcTermG t = tile[k];
         float s, c;
