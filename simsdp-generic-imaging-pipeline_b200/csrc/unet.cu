@@ -872,15 +872,16 @@ __global__ void __launch_bounds__(256) k_concat_up(int h, int w, int ca, int cb,
 // channels: the three column taps share its dz fragments, five ldmatrix per
 // twelve mma (with a warp per tap it was four per eight: a quarter of the
 // clocks each, 46 clocks per SM and eight mma where the tensor pipe alone
-// takes 17).  Partial sums are added to the FP32 gradients with atomics once
-// per CTA.
+// takes 17).
 // What is summed in one accumulator, and in which order, decides the rounding
 // of a gradient, and Adam turns the sign of a gradient near zero into a whole
 // step of the weight.  An accumulator therefore runs over all rows of its
 // tiles in order, and the number of CTAs per channel block is 4 per SM
 // whatever the kernel's occupancy: with the rows in two halves and another
 // number of CTAs the gradients of the 256-channel layer moved by 66 times what
-// two runs differ by.
+// two runs with float atomics differ by.  The CTAs' sums go to scratch, and
+// k_wgrad_sum adds them up in doubles and in one order, so that a training
+// step repeats bit for bit.
 // A thread stages the same places of every tile, so that its offsets from
 // the tile's origin are computed once.
 // 16 x 256^2, all 14 layers: 1737 -> 1517 us (32 -> 32 channels at level 0
@@ -891,7 +892,7 @@ struct WgradArgs {
     const bf16 *dz;  // [n][h][w][cout]
     int cout;
     VIn in;
-    float *dw;       // [9][cout][cin]
+    float *part;     // [CTA][9][32][32]
     int n, tiles_x, tiles_y, ntiles;
 };
 
@@ -900,6 +901,7 @@ constexpr int kWgX = 4 * kHalo * 16;         // input halo: 4 planes x 180 pixel
 constexpr int kWgStage = kWgDz + kWgX;
 constexpr int kWgBytes = 2 * kWgStage;
 constexpr int kWgThreads = 192;              // 3 row taps x 2 halves of the input channels
+constexpr int kWgBlock = 9 * 32 * 32;        // sums of one CTA
 
 __global__ void __launch_bounds__(kWgThreads, 4) k_wgrad3x3(WgradArgs p)
 {
@@ -1019,6 +1021,7 @@ __global__ void __launch_bounds__(kWgThreads, 4) k_wgrad3x3(WgradArgs p)
         }
     }
     const int g = lane >> 2, tq = lane & 3;
+    float *out = p.part + ((size_t)(blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * kWgBlock;
 #pragma unroll
     for (int dx = 0; dx < 3; ++dx)
 #pragma unroll
@@ -1026,24 +1029,125 @@ __global__ void __launch_bounds__(kWgThreads, 4) k_wgrad3x3(WgradArgs p)
 #pragma unroll
             for (int j = 0; j < 2; ++j)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int co = co0 + mt * 16 + g + (e >> 1) * 8;
-                    const int ci = ci0 + half * 16 + j * 8 + tq * 2 + (e & 1);
-                    atomicAdd(p.dw + ((size_t)(3 * dy + dx) * p.cout + co) * cin + ci, acc[dx][mt][j][e]);
+                for (int e = 0; e < 2; ++e) {
+                    const int co = mt * 16 + g + e * 8, ci = half * 16 + j * 8 + tq * 2;
+                    *reinterpret_cast<float2 *>(out + ((3 * dy + dx) * 32 + co) * 32 + ci) =
+                        make_float2(acc[dx][mt][j][2 * e], acc[dx][mt][j][2 * e + 1]);
                 }
 }
 
-// Bias gradient: db[c] += sum_p dz[p][c]; c divides 256 (32 .. 256 channels).
-// A thread sums the pixels of its chain in order and adds the result with one
-// atomic, the composition the weight gradient's comment asks for: sums taken
-// from the weight gradient's tiles, or chains joined before the atomics, move
-// the biases by as much as two runs differ by.  Bound by the latency of a
-// chain's loads, so 32 pixels' are in flight together: all 14 layers of
-// 16 x 256^2 394 us (520 with 16; as the compiler unrolled it 622).
+constexpr int kSumWarps = 16;  // per block of the kernels that add partial sums up
+
+// Loads from L2 that stay where they are written: the compiler otherwise moves
+// the loads of a batch down to their uses, one round trip after the other.
+__device__ __forceinline__ float4 ldcg_now(const float4 *p)
+{
+    float4 v;
+    asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double ldcg_now(const double *p)
+{
+    double v;
+    asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+
+// out[col] += the column's sum over `rows` rows of doubles, for the 32 columns
+// from col0 on.
+__device__ __forceinline__ void add_columns(const double *__restrict__ part, int rows, int cols, int col0, float *out)
+{
+    __shared__ double s_part[kSumWarps][32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, col = col0 + lane;
+    double a = 0.0;
+    if (col < cols)
+        for (int r0 = wid; r0 < rows; r0 += 16 * kSumWarps) {
+            double v[16];
+#pragma unroll
+            for (int k = 0; k < 16; ++k) v[k] = ldcg_now(part + (size_t)min(r0 + k * kSumWarps, rows - 1) * cols + col);
+#pragma unroll
+            for (int k = 0; k < 16; ++k) a += r0 + k * kSumWarps < rows ? v[k] : 0.0;
+        }
+    s_part[wid][lane] = a;
+    __syncthreads();
+    if (wid == 0 && col < cols) {
+        for (int k = 1; k < kSumWarps; ++k) a += s_part[k][lane];
+        out[col] = (float)((double)out[col] + a);
+    }
+}
+__global__ void __launch_bounds__(32 * kSumWarps) k_add_columns(const double *__restrict__ part, int rows, int cols, float *out)
+{
+    add_columns(part, rows, cols, 32 * blockIdx.x, out);
+}
+
+// Adds the sums of k_wgrad3x3's CTAs (z of each of the nbx x nby channel
+// blocks) to dw, and those of k_bias_grad's blocks to db.  A segment of 128
+// neighbouring sums is read by `share` warps, a part of the z's each, ten
+// loads in flight; the last cout / 32 blocks take the biases.  Bound by the
+// latency of reading 22 MB from L2: all 14 layers of 16 x 256^2 173 us
+// (305 where the compiler moved the loads to their uses).
+constexpr int kWgSegments = kWgBlock / 128;
+__global__ void __launch_bounds__(32 * kSumWarps) k_wgrad_sum(const float *__restrict__ part, int z, int share, int nbx, int nby,
+                                                              int cout, int cin, float *dw,
+                                                              const double *__restrict__ bpart, int brows, float *db)
+{
+    constexpr int U = 10;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int segments = nbx * nby * kWgSegments, per = kSumWarps / share;
+    const int blocks = (segments + per - 1) / per;
+    if ((int)blockIdx.x >= blocks) {
+        add_columns(bpart, brows, cout, 32 * ((int)blockIdx.x - blocks), db);
+        return;
+    }
+    __shared__ double s_sum[kSumWarps][128];
+    const int segment = blockIdx.x * per + wid / share, w = wid % share;
+    double a[4] = {};
+    if (segment < segments) {
+        const int z0 = w * z / share, z1 = (w + 1) * z / share;
+        const size_t step = (size_t)nbx * nby * kWgBlock;
+        const float *src = part + (size_t)segment * 128 + 4 * lane;
+        for (int k0 = z0; k0 < z1; k0 += U) {
+            float4 v[U];
+#pragma unroll
+            for (int k = 0; k < U; ++k) v[k] = ldcg_now(reinterpret_cast<const float4 *>(src + min(k0 + k, z1 - 1) * step));
+#pragma unroll
+            for (int k = 0; k < U; ++k)
+                if (k0 + k < z1) {
+                    a[0] += v[k].x;
+                    a[1] += v[k].y;
+                    a[2] += v[k].z;
+                    a[3] += v[k].w;
+                }
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) s_sum[wid][4 * lane + q] = a[q];
+    __syncthreads();
+    for (int t = threadIdx.x; t < 128 * per; t += 32 * kSumWarps) {
+        const int seg = blockIdx.x * per + (t >> 7);
+        if (seg >= segments) break;
+        double sum = 0.0;
+        for (int k = 0; k < share; ++k) sum += s_sum[(t >> 7) * share + k][t & 127];
+        const int blk = seg / kWgSegments, e = seg % kWgSegments * 128 + (t & 127), tap = e >> 10;
+        const int co = 32 * (blk % nbx) + ((e >> 5) & 31), ci = 32 * (blk / nbx) + (e & 31);
+        float *d = dw + ((size_t)tap * cout + co) * cin + ci;
+        *d = (float)((double)*d + sum);
+    }
+}
+
+// Bias gradient: sums of dz[p][c] over the pixels of a block, which k_wgrad_sum
+// adds to db; c divides 256 (32 .. 256 channels).  A thread sums the pixels of
+// its chain in order in FP32, the composition the weight gradient's comment
+// asks for (sums taken from the weight gradient's tiles moved the biases by as
+// much as two runs with atomics differ by); a block adds its chains up in
+// doubles.  Bound by the latency of a chain's loads, so 32 pixels' are in
+// flight together: all 14 layers of 16 x 256^2 363 us (490 with 16; as the
+// compiler unrolled it 622).
 constexpr int kBiasAhead = 32;
 __global__ void __launch_bounds__(256) k_bias_grad(const bf16 *__restrict__ dz, long long npix, int c,
-                                                  float *__restrict__ db)
+                                                  double *__restrict__ part)
 {
+    __shared__ float s_chain[256];
     const int rows = 256 / c;
     const int ch = threadIdx.x % c, r0 = threadIdx.x / c;
     const long long first = (long long)blockIdx.x * rows + r0, step = (long long)gridDim.x * rows;
@@ -1058,7 +1162,13 @@ __global__ void __launch_bounds__(256) k_bias_grad(const bf16 *__restrict__ dz, 
 #pragma unroll
         for (int u = 0; u < kBiasAhead; ++u) s += __bfloat162float(v[u]);
     }
-    atomicAdd(db + ch, s);
+    s_chain[threadIdx.x] = s;
+    __syncthreads();
+    if ((int)threadIdx.x < c) {
+        double t = 0.0;
+        for (int r = 0; r < rows; ++r) t += s_chain[r * c + threadIdx.x];
+        part[(size_t)blockIdx.x * c + threadIdx.x] = t;
+    }
 }
 
 // ----------------------------------------------------------------------------
@@ -1190,22 +1300,19 @@ __global__ void k_head_fwd(long long npix, long long pix_per_img, int c, const b
     }
 }
 
-// dd0[p][c] = go[p] * bf16(hw[c]) * (d0[p][c] > 0); dhw[c] += sum_p go[p] d0[p][c];
-// dhb += sum_p go[p].  Four threads per pixel, eight channels each, so that
-// the sums stay in registers (one thread per pixel kept them in local
+// dd0[p][c] = go[p] * bf16(hw[c]) * (d0[p][c] > 0), and per block the sums
+// go[p] d0[p][c] and go[p], which k_add_columns adds to the head's gradients.
+// Four threads per pixel, eight channels each, so that the sums stay in registers (one thread per pixel kept them in local
 // memory: 96 us for 16 x 256^2, now 36).  A warp takes 32 consecutive pixels
 // at a time; the chain of a pixel's place in the warp runs over all of the
 // warp's pixel groups, and the 32 chains are summed as a tree: over pixels 16
 // and 8 apart in the thread, then 4, 2 and 1 apart by shuffles.
 __global__ void __launch_bounds__(256) k_head_bwd(long long npix, const bf16 *__restrict__ d0,
                                                  const float *__restrict__ hw, const float *__restrict__ go,
-                                                 bf16 *__restrict__ dd0, float *__restrict__ dhw,
-                                                 float *__restrict__ dhb)
+                                                 bf16 *__restrict__ dd0, double *__restrict__ sums)
 {
     constexpr int C = 32;  // channels of the last layer
-    __shared__ float s_dw[C + 1];
-    for (int i = threadIdx.x; i <= C; i += blockDim.x) s_dw[i] = 0.f;
-    __syncthreads();
+    __shared__ float s_warp[8][C + 1];
     const int lane = threadIdx.x & 31, g8 = lane & 3;
     float wv[8], part[4][8], pb[4];
 #pragma unroll
@@ -1246,14 +1353,17 @@ __global__ void __launch_bounds__(256) k_head_bwd(long long npix, const bf16 *__
     for (int e = 0; e < 8; ++e) {
         float v = (part[0][e] + part[2][e]) + (part[1][e] + part[3][e]);
         for (int off = 16; off >= 4; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-        if (lane < 4) atomicAdd(&s_dw[8 * g8 + e], v);
+        if (lane < 4) s_warp[threadIdx.x >> 5][8 * g8 + e] = v;
     }
     float b = (pb[0] + pb[2]) + (pb[1] + pb[3]);
     for (int off = 16; off >= 4; off >>= 1) b += __shfl_xor_sync(0xffffffffu, b, off);
-    if (lane == 0) atomicAdd(&s_dw[C], b);
+    if (lane == 0) s_warp[threadIdx.x >> 5][C] = b;
     __syncthreads();
-    for (int k = threadIdx.x; k < C; k += blockDim.x) atomicAdd(dhw + k, s_dw[k]);
-    if (threadIdx.x == 0) atomicAdd(dhb, s_dw[C]);
+    if (threadIdx.x <= C) {
+        double t = 0.0;
+        for (int k = 0; k < 8; ++k) t += s_warp[k][threadIdx.x];
+        sums[(size_t)blockIdx.x * (C + 1) + threadIdx.x] = t;
+    }
 }
 
 // BF16 copies of all layers' FP32 weights, in one launch (blockIdx.y: the
@@ -1410,6 +1520,8 @@ struct sdp_unet {
     // gradient scratch (training)
     bf16 *gz[kLevels][2] = {};
     bf16 *dcat[kLevels - 1] = {};
+    float *wpart = nullptr;    // the CTAs' weight-gradient sums
+    double *cpart = nullptr;   // the blocks' bias and head sums
     bf16 *cat[kLevels - 1] = {};  // [e_l, up(low)] materialised for the tensor-core path
     // shape of the last forward pass
     int n = 0, h = 0, w = 0;
@@ -1620,24 +1732,34 @@ int conv(const sdp_unet *u, VIn in, const bf16 *wk, const bf16 *wtc, const float
     return SDP_OK;
 }
 
-int wgrad(const bf16 *dz, int cout, VIn in, float *dw, float *db, int n, cudaStream_t st)
+// Scratch of the gradient sums: the CTAs' weight sums, and the bias or head
+// sums of at most grid_for's blocks.
+size_t wgrad_part_floats() { return (size_t)(4 * num_sms() + 64) * kWgBlock; }  // 64: channel blocks of the widest layer
+size_t column_part_doubles() { return (size_t)num_sms() * 16 * 256; }
+
+int wgrad(const sdp_unet *u, const bf16 *dz, int cout, VIn in, float *dw, float *db, int n, cudaStream_t st)
 {
     WgradArgs a;
     a.dz = dz;
     a.cout = cout;
     a.in = in;
-    a.dw = dw;
+    a.part = u->wpart;
     a.n = n;
     a.tiles_x = (in.w + kTW - 1) / kTW;
     a.tiles_y = (in.h + kTH - 1) / kTH;
     a.ntiles = (int)tiles(n, in.h, in.w);
-    const int cin = in.ca + in.cb;
-    const int blocks_xy = (cout / 32) * (cin / 32);
-    const int z = std::max(1, std::min(a.ntiles, (4 * num_sms() + blocks_xy - 1) / blocks_xy));
-    k_wgrad3x3<<<dim3(cout / 32, cin / 32, z), kWgThreads, kWgBytes, st>>>(a);
+    const int cin = in.ca + in.cb, nbx = cout / 32, nby = cin / 32;
+    const int z = std::max(1, std::min(a.ntiles, (4 * num_sms() + nbx * nby - 1) / (nbx * nby)));
+    k_wgrad3x3<<<dim3(nbx, nby, z), kWgThreads, kWgBytes, st>>>(a);
     SDP_LAUNCH_CHECK();
     const long long np = (long long)n * in.h * in.w;
-    k_bias_grad<<<grid_for(np / (256 / cout) + 1), 256, 0, st>>>(dz, np, cout, db);
+    const int blocks = grid_for(np / (256 / cout) + 1);
+    k_bias_grad<<<blocks, 256, 0, st>>>(dz, np, cout, u->cpart);
+    SDP_LAUNCH_CHECK();
+    const int share = z >= 128 ? 16 : z >= 32 ? 8 : 4;
+    const int per = kSumWarps / share, segments = nbx * nby * kWgSegments;
+    k_wgrad_sum<<<(segments + per - 1) / per + nbx, 32 * kSumWarps, 0, st>>>(u->wpart, z, share, nbx, nby, cout, cin, dw,
+                                                                            u->cpart, blocks, db);
     SDP_LAUNCH_CHECK();
     return SDP_OK;
 }
@@ -1746,6 +1868,8 @@ SDP_EXPORT int sdp_unet_create(sdp_unet **out, int base_channels, int in_channel
         }
         for (int l = 0; l < kLevels - 1; ++l) o_dcat[l] = take(pix(u, l) * (ch(u, l) + ch(u, l + 1)) * 2);
     }
+    const size_t o_wpart = u->training ? take(wgrad_part_floats() * sizeof(float)) : 0;
+    const size_t o_cpart = u->training ? take(column_part_doubles() * sizeof(double)) : 0;
     void *arena = nullptr;
     cudaError_t e = cudaMalloc(&arena, bytes);
     if (e != cudaSuccess) {
@@ -1760,6 +1884,8 @@ SDP_EXPORT int sdp_unet_create(sdp_unet **out, int base_channels, int in_channel
         u->grad = reinterpret_cast<float *>(A + o_grad);
         u->adam_m = reinterpret_cast<float *>(A + o_m);
         u->adam_v = reinterpret_cast<float *>(A + o_v);
+        u->wpart = reinterpret_cast<float *>(A + o_wpart);
+        u->cpart = reinterpret_cast<double *>(A + o_cpart);
     }
     for (int k = 0; k < kLayers; ++k) {
         u->layer[k].w = reinterpret_cast<bf16 *>(A + o_w[k]);
@@ -1975,21 +2101,22 @@ SDP_EXPORT int sdp_unet_backward(sdp_unet *u, const float *grad_output, void *st
     float *G = u->grad;
     const int c0 = ch(u, 0);
     // head: dZ(d0) -> gz[0][0]
-    k_head_bwd<<<grid_for(np), 256, 0, st>>>(
-        np, u->d[0][1], u->master + u->head_off, grad_output, u->gz[0][0], G + u->head_off, G + u->head_off + c0);
+    k_head_bwd<<<grid_for(np), 256, 0, st>>>(np, u->d[0][1], u->master + u->head_off, grad_output, u->gz[0][0], u->cpart);
+    SDP_LAUNCH_CHECK();
+    k_add_columns<<<(c0 + 32) / 32, 32 * kSumWarps, 0, st>>>(u->cpart, grid_for(np), c0 + 1, G + u->head_off);
     SDP_LAUNCH_CHECK();
     // decoder, top (level 0) down to level kLevels - 2; gz[l][0] holds dZ of d_l on entry
     for (int l = 0; l <= kLevels - 2; ++l) {
         const int hl = h >> l, wl = w >> l, c = ch(u, l), c1 = ch(u, l + 1);
         const Layer &La = u->layer[dec_layer(l, 0)], &Lb = u->layer[dec_layer(l, 1)];
         // second conv: d_l = conv(d_l a)
-        SDP_TRY(wgrad(u->gz[l][0], c, vin(u->d[l][0], c, nullptr, 0, hl, wl), G + Lb.woff, G + Lb.boff, n, st));
+        SDP_TRY(wgrad(u, u->gz[l][0], c, vin(u->d[l][0], c, nullptr, 0, hl, wl), G + Lb.woff, G + Lb.boff, n, st));
         SDP_TRY(conv(u, vin(u->gz[l][0], c, nullptr, 0, hl, wl), Lb.wt, Lb.wttc, nullptr, u->d[l][0], u->gz[l][1],
                      c, 0, n,
                      st));
         // first conv: d_l a = conv([e_l, up(low)])
         const bf16 *low = (l == kLevels - 2) ? u->e[l + 1][1] : u->d[l + 1][1];
-        SDP_TRY(wgrad(u->gz[l][1], c, vin(u->e[l][1], c, low, c1, hl, wl), G + La.woff, G + La.boff, n, st));
+        SDP_TRY(wgrad(u, u->gz[l][1], c, vin(u->e[l][1], c, low, c1, hl, wl), G + La.woff, G + La.boff, n, st));
         SDP_TRY(conv(u, vin(u->gz[l][1], c, nullptr, 0, hl, wl), La.wt, La.wttc, nullptr, nullptr, u->dcat[l],
                      c + c1, 0, n,
                      st));
@@ -2002,13 +2129,13 @@ SDP_EXPORT int sdp_unet_backward(sdp_unet *u, const float *grad_output, void *st
     for (int l = kLevels - 1; l >= 0; --l) {
         const int hl = h >> l, wl = w >> l, c = ch(u, l);
         const Layer &La = u->layer[enc_layer(l, 0)], &Lb = u->layer[enc_layer(l, 1)];
-        SDP_TRY(wgrad(u->gz[l][0], c, vin(u->e[l][0], c, nullptr, 0, hl, wl), G + Lb.woff, G + Lb.boff, n, st));
+        SDP_TRY(wgrad(u, u->gz[l][0], c, vin(u->e[l][0], c, nullptr, 0, hl, wl), G + Lb.woff, G + Lb.boff, n, st));
         SDP_TRY(conv(u, vin(u->gz[l][0], c, nullptr, 0, hl, wl), Lb.wt, Lb.wttc, nullptr, u->e[l][0], u->gz[l][1],
                      c, 0, n,
                      st));
         const bf16 *src = l == 0 ? u->x : u->pool[l];
         const int cs = l == 0 ? kInPad : ch(u, l - 1);
-        SDP_TRY(wgrad(u->gz[l][1], c, vin(src, cs, nullptr, 0, hl, wl), G + La.woff, G + La.boff, n, st));
+        SDP_TRY(wgrad(u, u->gz[l][1], c, vin(src, cs, nullptr, 0, hl, wl), G + La.woff, G + La.boff, n, st));
         if (l == 0) break;
         // data gradient of the pooled input (cs channels at level l), into gz[l][0]
         SDP_TRY(conv(u, vin(u->gz[l][1], c, nullptr, 0, hl, wl), La.wt, La.wttc, nullptr, nullptr, u->gz[l][0],

@@ -2,7 +2,7 @@
 zero takes its sign from the rounding of its sum, and Adam turns that sign
 into a whole step of the weight, so the sums keep their composition: chains
 over all rows of a tile in order, the same tiles in one chain, the same pixels
-in a chain of a bias or head sum.  The recorded gradients
+in a chain of a bias or head sum, and meet in one order.  The recorded gradients
 (golden/unet_grads.npz) are those of the kernels with one warp per tap and one
 thread per chain; `python tests/test_gpu_unet_sums.py FILE` on a GPU writes
 the present ones.
@@ -70,6 +70,55 @@ def test_sums_keep_their_composition(sdp, device):
             d = got[k].astype(np.float64) - ref[k]
             rel = np.sqrt(np.mean(d ** 2) / np.mean(ref[k].astype(np.float64) ** 2))
             assert rel <= bound, (k, rel)
+
+
+def test_steps_repeat_bit_for_bit(sdp, device):
+    """Three training steps from one state, twice: no sum depends on the order
+    in which CTAs finish."""
+    import torch
+    import unet_ref as U
+    rng = np.random.default_rng(5)
+    p = U.init_params(32, 3, rng)
+    n, size = 4, 128
+    x = torch.from_numpy(rng.standard_normal((n, 3, size, size)).astype(np.float32)).cuda()
+    target = torch.from_numpy(rng.standard_normal((n, size, size)).astype(np.float32)).cuda()
+    runs = []
+    for _ in range(2):
+        net = sdp.UNet(sdp.load(), 3, n, size, size)
+        net.set_params(p)
+        out, grad = torch.empty((n, size, size), device="cuda"), torch.empty((n, size, size), device="cuda")
+        scratch, loss = torch.empty(2 * n * size * size, device="cuda"), torch.zeros(1, dtype=torch.float64, device="cuda")
+        seen = []
+        for _ in range(3):
+            net.forward(x, out)
+            device.blur_mse(out, target, scratch, grad, loss)
+            net.zero_grads()
+            net.backward(grad)
+            net.adam_step(1e-3)
+            seen += [out.cpu().numpy(), net.get_grads(), net.get_params()]
+        net.close()
+        runs.append(seen)
+    for a, b in zip(*runs):
+        np.testing.assert_array_equal(a, b)
+
+
+def test_gradients_accumulate(sdp, device):
+    """A second backward pass adds to the gradients of the first."""
+    import torch
+    import unet_ref as U
+    rng = np.random.default_rng(6)
+    net = sdp.UNet(sdp.load(), 3, 2, 64, 64)
+    net.set_params(U.init_params(32, 3, rng))
+    x = torch.from_numpy(rng.standard_normal((2, 3, 64, 64)).astype(np.float32)).cuda()
+    go = torch.from_numpy(rng.standard_normal((2, 64, 64)).astype(np.float32)).cuda()
+    net.forward(x, torch.empty((2, 64, 64), device="cuda"))
+    net.zero_grads()
+    net.backward(go)
+    once = net.get_grads()
+    net.backward(go)
+    twice = net.get_grads()
+    net.close()
+    np.testing.assert_allclose(twice, 2 * once, rtol=2.0 ** -22, atol=0)
 
 
 if __name__ == "__main__":
